@@ -1,26 +1,24 @@
-"""ctypes binding of libdsv32_b200.so (the C ABI declared in include/dsv32_b200.h).
+"""ctypes binding of libdsv32_b200.so (the C ABI declared in include/dsv32_b200.h) and of the native front end _front.so.
 
-There is no CPU fallback: if the shared library is missing or a call is rejected the
-functions here raise.
+Both are required and neither is touched before load(): the package can be imported, and its Python parts used, where they
+have not been built.  There is no CPU fallback: if one of them is missing or a call is rejected the functions here raise.
 """
 from __future__ import annotations
 
 import ctypes as C
+import importlib
 import os
 
-import torch  # noqa: F401  (the native front end links against torch's libraries)
 
-try:
-    from . import _front as front
-except ImportError as e:
-    class _NoFront:
-        """Stands in for a front end that has not been built: declines every call; load() then says what is missing."""
-        error = e
+class _NotLoaded:
+    """The front end until load() has replaced it: declines every call, so that the Python layer takes it and calls load()."""
 
-        def __getattr__(self, name):
-            return lambda *args: None
+    def __getattr__(self, name):
+        return lambda *args: None
 
-    front = _NoFront()
+
+front = _NotLoaded()
+_status_words = {}   # device index -> address: load() passes on those made before it
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("DSV32_B200_LIB", os.path.join(HERE, "libdsv32_b200.so"))
@@ -246,9 +244,19 @@ class Dsv32Error(RuntimeError):
     """A call into libdsv32_b200.so was rejected (host-side validation or CUDA launch error)."""
 
 
+def _import_front():
+    import torch  # noqa: F401  (its libraries come first: the front end links against them)
+    importlib.invalidate_caches()   # the file may have been built by this very process
+    try:
+        return importlib.import_module("._front", __package__)
+    except ImportError as e:
+        raise Dsv32Error(f"the native front end (_front.so) cannot be imported: {e}; "
+                         "build it with `python -m pypto_b200.build`") from e
+
+
 def load():
-    """Load the shared library (once).  Raises if it has not been built."""
-    global _lib
+    """Load the shared library and the front end (once).  Raises if either has not been built."""
+    global _lib, front
     if _lib is not None:
         return _lib
     if not os.path.exists(LIB_PATH):
@@ -261,12 +269,18 @@ def load():
         fn.argtypes = args
     if lib.dsv32_abi_version() != ABI_VERSION:
         raise Dsv32Error(f"ABI mismatch: library {lib.dsv32_abi_version()}, binding {ABI_VERSION}")
-    if hasattr(front, "error"):
-        raise Dsv32Error(f"the native front end (_front.so) cannot be imported: {front.error}; "
-                         "build it with `python -m pypto_b200.build`")
-    front.bind({name: C.cast(getattr(lib, name), c_void_p).value for name in EXPORTS}, check)
-    _lib = lib
+    native = _import_front()
+    native.bind({name: C.cast(getattr(lib, name), c_void_p).value for name in EXPORTS}, check)
+    _lib, front = lib, native
+    for index, address in list(_status_words.items()):
+        native.set_status(index, address)
     return lib
+
+
+def set_status(index: int, address: int):
+    """The status word of a device, for the calls that the front end takes."""
+    _status_words[index] = address
+    front.set_status(index, address)
 
 
 def check(rc: int, what: str):

@@ -132,7 +132,7 @@ def status_word(device):
     if st is None:
         st = torch.zeros(4, dtype=torch.int32, device=device)
         _STATUS[key] = st
-        _lib.front.set_status(key[1], st.data_ptr())
+        _lib.set_status(key[1], st.data_ptr())
     return st
 
 
