@@ -254,7 +254,7 @@ proj_tc_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant_
 
 // ---- host ------------------------------------------------------------------------------------------------------------
 // Column tile and split of the reduction for a product of t tokens, `cols` output columns and `k_chunks` reduction chunks.
-ProjPlan proj_plan(int t, int cols, int k_chunks) {
+ProjPlan proj_plan(int t, int cols, int k_chunks, int ctas) {
   ProjPlan pl;
   pl.wide = t > 128;
   const int kn = pl.wide ? 256 : 128;
@@ -263,9 +263,12 @@ ProjPlan proj_plan(int t, int cols, int k_chunks) {
   int s = sm_count() / (pl.m_tiles * pl.n_tiles);
   // every split costs a write and a read of the partial sums, and below four chunks a CTA does not fill its ring
   s = s < k_chunks / 4 ? s : k_chunks / 4;
-  pl.splits = s < 1 ? 1 : (s > 16 ? 16 : s);
+  s = s < 1 ? 1 : (s > 16 ? 16 : s);
   const int seg = (k_chunks + kProjSegChunks - 1) / kProjSegChunks;
-  pl.segments = seg > pl.splits ? seg : pl.splits;
+  pl.segments = seg > s ? seg : s;
+  // (fewer CTAs take the same segments, several each: how the sum is cut, and with it its error, does not depend on them)
+  const int fit = ctas / (pl.m_tiles * pl.n_tiles);
+  pl.splits = ctas <= 0 || s <= fit ? s : (fit < 1 ? 1 : fit);
   return pl;
 }
 
@@ -283,7 +286,7 @@ static int launch_proj(const ProjPlan& pl, const CUtensorMap& a, const CUtensorM
 
 // partial [splits][t][ldc] fp32 with ldc = proj_ld(columns of all segments); rows of x and w multiples of 16 bytes.
 int launch_proj_bf16(const __nv_bfloat16* x, int t, int k, const ProjSegment* segs, int nsegs, bool k_major, float* partial,
-                     uint32_t* status, cudaStream_t stream) {
+                     uint32_t* status, cudaStream_t stream, int ctas) {
   if (t <= 0) return DSV32_OK;
   ProjParams p{};
   p.status = status;
@@ -300,7 +303,7 @@ int launch_proj_bf16(const __nv_bfloat16* x, int t, int k, const ProjSegment* se
     else rc = make_tensor_map_2d_u8(&b[i], s.w, k, static_cast<uint64_t>(s.cols) * 2, 64, 128);
   }
   const int ldc = p.n_chunks * 64;
-  const ProjPlan pl = proj_plan(t, ldc, p.k_chunks);
+  const ProjPlan pl = proj_plan(t, ldc, p.k_chunks, ctas);
   if (rc == DSV32_OK) rc = make_tensor_map_3d_u8(&c, partial, pl.splits, t, static_cast<uint64_t>(ldc) * 4, 32);
   if (rc != DSV32_OK) return rc;
   p.m_tiles = pl.m_tiles; p.n_tiles = pl.n_tiles; p.splits = pl.splits; p.segments = pl.segments;

@@ -451,11 +451,11 @@ heads_tc_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant
 }
 
 template <bool kV4>
-static int launch_heads(const CUtensorMap (&maps)[7], const HeadParams& p, cudaStream_t stream) {
+static int launch_heads(const CUtensorMap (&maps)[7], const HeadParams& p, cudaStream_t stream, int ctas = 0) {
   auto kernel = heads_tc_kernel<kV4>;
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kHdSmemBytes));
-  const int sms = sm_count();
-  launch_ex(kernel, dim3(p.items < sms ? p.items : sms), kHdThreads, kHdSmemBytes, stream, true, 1, maps[0], maps[1], maps[2], maps[3],
+  if (ctas <= 0) ctas = sm_count();
+  launch_ex(kernel, dim3(p.items < ctas ? p.items : ctas), kHdThreads, kHdSmemBytes, stream, true, 1, maps[0], maps[1], maps[2], maps[3],
             maps[4], maps[5], maps[6], p);
   count_launch();
   return check_launch("heads_tc_kernel");
@@ -463,7 +463,7 @@ static int launch_heads(const CUtensorMap (&maps)[7], const HeadParams& p, cudaS
 
 // The heads of the V3.2 prologs: MLA heads (m given), indexer heads (ip given), or both, which then share t and q_norm.
 // Launched dependent on the kernel before it in the stream; `independent`: q_norm is not that kernel's output.
-int launch_prolog_heads(const MlaParams* m, const PrologParams* ip, bool independent, cudaStream_t stream) {
+int launch_prolog_heads(const MlaParams* m, const PrologParams* ip, bool independent, cudaStream_t stream, int ctas) {
   HeadParams p{};
   p.t = m != nullptr ? m->t : ip->t;
   p.m_tiles = (p.t + 127) / 128;
@@ -503,7 +503,7 @@ int launch_prolog_heads(const MlaParams* m, const PrologParams* ip, bool indepen
     if (m == nullptr) maps[i] = maps[0];
   for (int i = 5; i < 7; ++i)
     if (ip == nullptr) maps[i] = maps[0];
-  return launch_heads<false>(maps, p, stream);
+  return launch_heads<false>(maps, p, stream, ctas);
 }
 
 // The query heads of the V4 indexer prolog.

@@ -172,7 +172,8 @@ struct MlaParams {
 // The V3.2 prologs: the MLA half, the indexer half, or both on one x (partial: prolog_partial_bytes)
 int launch_prolog_v32(const MlaParams* m, const PrologParams* ip, float* partial, cudaStream_t stream);
 size_t prolog_partial_bytes(int t, bool mla, bool indexer);
-int launch_prolog_heads(const MlaParams* m, const PrologParams* ip, bool independent, cudaStream_t stream);   // heads_tc.cu
+// heads_tc.cu; ctas: CTAs that share the items, 0 = one per SM
+int launch_prolog_heads(const MlaParams* m, const PrologParams* ip, bool independent, cudaStream_t stream, int ctas = 0);
 int launch_prolog_v4_heads(const PrologParams& ip, cudaStream_t stream);
 // Projections (gemm_tc.cu): fp32 partial sums [splits][t][proj_ld(columns)] of x[t, k] times up to four weight matrices side
 // by side, each starting at a multiple of 64 columns; weights [k, cols] or with k_major [cols, k], rows of 16-byte multiples.
@@ -185,10 +186,10 @@ struct ProjPlan {
   int m_tiles, n_tiles, splits, segments;
 };
 inline int proj_ld(int cols) { return (cols + 63) / 64 * 64; }
-ProjPlan proj_plan(int t, int cols, int k_chunks);
+ProjPlan proj_plan(int t, int cols, int k_chunks, int ctas = 0);   // ctas: CTAs the product may take, 0 = one per SM
 size_t proj_partial_bytes(int t, int k, int cols);
 int launch_proj_bf16(const __nv_bfloat16* x, int t, int k, const ProjSegment* segs, int nsegs, bool k_major, float* partial,
-                     uint32_t* status, cudaStream_t stream);
+                     uint32_t* status, cudaStream_t stream, int ctas = 0);
 // C[t, n] (fp32 or bf16) = A[t, k] x B (bf16; B as [k, n], or with b_kmajor as [n, k]) through partial sums in `workspace`
 int launch_bf16_gemm(const __nv_bfloat16* a, int t, int k, const __nv_bfloat16* b, int n, bool b_kmajor, void* out,
                      bool out_bf16, void* workspace, uint32_t* status, cudaStream_t stream);

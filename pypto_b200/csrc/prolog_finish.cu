@@ -257,9 +257,8 @@ __global__ void __launch_bounds__(256) prolog_finish_rows_kernel(PrologFinishPar
   }
 }
 
-static int launch_prolog_finish(const PrologFinishParams& p, int nsections, cudaStream_t stream) {
-  // a CTA per token while that many run at once (three sections of 512 threads on every SM), a warp per token beyond
-  if (p.t <= 192) launch_ex(prolog_finish_kernel, dim3(p.t, nsections), kFinThreads, 0, stream, true, 1, p);
+static int launch_prolog_finish(const PrologFinishParams& p, int nsections, bool rows, cudaStream_t stream) {
+  if (!rows) launch_ex(prolog_finish_kernel, dim3(p.t, nsections), kFinThreads, 0, stream, true, 1, p);
   else launch_ex(prolog_finish_rows_kernel, dim3((p.t + 7) / 8, nsections), 256, 0, stream, true, 1, p);
   count_launch();
   return check_launch("prolog_finish_kernel");
@@ -268,6 +267,36 @@ static int launch_prolog_finish(const PrologFinishParams& p, int nsections, cuda
 // Workspace of the projections of either or both halves.
 size_t prolog_partial_bytes(int t, bool mla, bool indexer) {
   return t <= 0 ? 0 : proj_partial_bytes(t, 7168, (mla ? 2112 : 0) + (indexer ? 192 : 0));
+}
+
+// How the indexer prolog on its own runs: its heads take q_norm as an input, so they can run beside projection and finish.  A
+// heads CTA needs an SM to itself (200 KB of shared memory, 53,760 registers), and a finish CTA that was launched early and waits
+// for the projection keeps it from one: with the finish always before the heads the call went from 16.7 to 22.5 us where a CTA
+// per token and 64 heads' CTAs no longer fit the SMs.  Three forms in which nothing waits for an SM:
+//   finish, heads; a CTA per token          while finish and heads CTAs fit
+//   finish, heads; a warp per token         while projection, finish and heads CTAs fit
+//   heads, finish; a CTA per token          while the heads make at most two rounds: they take the CTAs of whole rounds, the
+//                                           projection the SMs they leave, in no more splits than it needs to be done with them
+// us at 64, 128, 192, 256, 384 and 512 tokens, everything read from memory:   16.4  18.5  20.2  20.5  28.0  28.8
+//   the finish always before the heads                                        16.2  24.4  26.7  29.2  30.8  37.1
+//   the heads on a second stream                                              18.6  20.9  22.9  25.9  28.8  36.7
+// Beyond that every kernel fills the chip by itself (1024 tokens: 45 us in the first order, 62 on two streams).
+struct IndexerPlan {
+  bool finish_rows, finish_last;
+  int proj_ctas, head_ctas;   // 0: one per SM
+};
+static IndexerPlan plan_indexer(int t) {
+  const int sms = sm_count(), m_tiles = (t + 127) / 128, items = 64 * m_tiles, rounds = (items + sms - 1) / sms;
+  IndexerPlan pl{t > 192, false, 0, 0};
+  if (rounds > 2 || t + items <= sms) return pl;
+  const ProjPlan proj = proj_plan(t, 192, 7168 / 64);
+  pl.finish_rows = proj.m_tiles * proj.n_tiles * proj.splits + (t + 7) / 8 + items <= sms;
+  if (pl.finish_rows) return pl;
+  pl.finish_last = true;
+  pl.head_ctas = (items + rounds - 1) / rounds;
+  const int room = sms - pl.head_ctas, most = proj.m_tiles * proj.n_tiles * (10 / rounds);
+  pl.proj_ctas = room < most ? room : most;
+  return pl;
 }
 
 // The V3.2 prologs: x times all weight matrices that take it (one launch), their finish (one), the heads (one).
@@ -284,13 +313,16 @@ int launch_prolog_v32(const MlaParams* m, const PrologParams* ip, float* partial
     segs[n++] = {ip->wk, 128};
     segs[n++] = {ip->w_proj, 64};
   }
-  int rc = launch_proj_bf16(m != nullptr ? m->x : ip->x, t, 7168, segs, n, false, partial, m != nullptr ? m->status : ip->status, stream);
+  // with the MLA half a CTA per token while that many run at once (three sections of 512 threads on every SM)
+  const IndexerPlan plan = m == nullptr ? plan_indexer(t) : IndexerPlan{t > 192, false, 0, 0};
+  int rc = launch_proj_bf16(m != nullptr ? m->x : ip->x, t, 7168, segs, n, false, partial, m != nullptr ? m->status : ip->status, stream,
+                            plan.proj_ctas);
   if (rc != DSV32_OK) return rc;
   PrologFinishParams f{};
   f.partial = partial;
   f.t = t;
   f.ld = (m != nullptr ? 2112 : 0) + (ip != nullptr ? 192 : 0);
-  f.splits = proj_plan(t, f.ld, 7168 / 64).splits;
+  f.splits = proj_plan(t, f.ld, 7168 / 64, plan.proj_ctas).splits;
   n = 0;
   if (m != nullptr) {
     f.sections[n++] = 0;
@@ -312,9 +344,10 @@ int launch_prolog_v32(const MlaParams* m, const PrologParams* ip, float* partial
     f.idx_cache = ip->k_cache; f.idx_scale_cache = ip->k_scale_cache; f.weights = ip->weights;
     f.status_idx = ip->status;
   }
-  rc = launch_prolog_finish(f, n, stream);
-  if (rc != DSV32_OK) return rc;
-  return launch_prolog_heads(m, ip, m == nullptr, stream);
+  if (!plan.finish_last) rc = launch_prolog_finish(f, n, plan.finish_rows, stream);
+  if (rc == DSV32_OK) rc = launch_prolog_heads(m, ip, m == nullptr, stream, plan.head_ctas);
+  if (rc == DSV32_OK && plan.finish_last) rc = launch_prolog_finish(f, n, plan.finish_rows, stream);
+  return rc;
 }
 
 }  // namespace dsv32

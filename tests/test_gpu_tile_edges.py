@@ -27,6 +27,32 @@ def test_fused_prolog_tiles(t):
     parity.test_mla_indexer_prolog_seeded_vs_oracle(t)
 
 
+# the indexer prolog on its own: the last and first token counts of the orders in which its kernels are launched and share the SMs.
+# With this many values some bf16 roundings fall the other way (2e-4 of the weights, at any of these counts): a weight, or the
+# maximum that a scale is, then differs by one step of bf16, 2^-7 of itself at most, and by the fp16 rounding after it.  A weight
+# near zero keeps the absolute error of its 7168-long sum: the 2.5e-5 of test_gpu_parity.py.
+@pytest.mark.parametrize("t", [84, 85, 128, 129, 193, 257, 385, 513])
+def test_indexer_prolog_orders(t, monkeypatch):
+    def check(got, ref, cache_index):
+        for name, a, b in zip(("q_int8", "q_scale", "k", "k_scale", "weights"), got, ref):
+            a, b = a.double().reshape(-1), b.double().reshape(-1)
+            diff = (a - b).abs()
+            if name in ("q_int8", "k"):
+                assert diff.max() <= 1, name
+                share, allowed = (diff > 0).double().mean().item(), 0.02
+            else:
+                assert bool((diff <= (2.0 ** -7 + 2.0 ** -10) * b.abs() + 2.5e-5).all()), name
+                share, allowed = (diff > 2.0 ** -10 * b.abs()).double().mean().item(), 0.01
+            print(f"[indexer prolog t={t}] {name}: {share:.1e} of the values differ")
+            assert share <= allowed, (name, share)
+        others = torch.ones(got[2].numel() // 128, dtype=torch.bool)
+        others[cache_index] = False
+        assert torch.equal(got[2].reshape(-1, 128)[others], ref[2].reshape(-1, 128)[others])
+
+    monkeypatch.setattr(parity, "_assert_prolog_close", check)
+    parity.test_prolog_config1_distributions_vs_oracle(t)
+
+
 # an odd number of (head, token tile) items, a hidden size that is not a multiple of a reduction chunk
 @pytest.mark.parametrize("t,heads,h", [(128, 3, 1000), (129, 3, 1000), (193, 2, 64), (257, 5, 1024)])
 @pytest.mark.parametrize("quant", [True, False])
