@@ -21,6 +21,8 @@
 // after scan 1).
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "kernels.cuh"
 #include "tc_common.cuh"
 
@@ -285,7 +287,10 @@ __device__ __forceinline__ bool small_row(const float* srow, int n, uint32_t idb
   return true;
 }
 
-__global__ void __launch_bounds__(kTopkThreads) topk_select_kernel(TopkParams p, int csize, int small) {
+// kSmall: every row of the launch has at most kSmallRow entries, of position ids.  kCtas: CTAs that share an SM, which sets the
+// registers: 64 a thread without spills where a CTA has an SM to itself, 32 (44 bytes of spills) where two hide each other's latencies.
+template <bool kSmall, int kCtas>
+__global__ void __launch_bounds__(kTopkThreads, kCtas) topk_select_kernel(TopkParams p, int csize) {
   extern __shared__ __align__(16) unsigned char topk_smem[];
   uint32_t* hist = reinterpret_cast<uint32_t*>(topk_smem);
   uint64_t* sel = reinterpret_cast<uint64_t*>(topk_smem + kHistBins * 4);
@@ -336,7 +341,7 @@ __global__ void __launch_bounds__(kTopkThreads) topk_select_kernel(TopkParams p,
     return true;
   };
 
-  if (small && n > 0) {   // (every row of the launch has at most kSmallRow entries)
+  if (kSmall && n > 0) {
     __syncthreads();
     if (small_row(srow, n, idb, p.k, orow, osrow, hist, sel, warp_tot, &s_kmin, &s_kmax, &s_maxgroup)) return;
     __syncthreads();
@@ -634,9 +639,20 @@ __global__ void __launch_bounds__(kTopkThreads) topk_select_kernel(TopkParams p,
   }
 }
 
+static int l2_bytes() {   // of the current device
+  static std::atomic<int> sizes[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = sizes[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrL2CacheSize, dev) != cudaSuccess || n <= 0) n = 1;
+    sizes[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 int launch_topk(const TopkParams& p, int rows, cudaStream_t stream) {
   if (rows <= 0) return DSV32_OK;
-  cudaFuncSetAttribute(topk_select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopkClusterSmemBytes);
   // A cluster per row while rows are few: the largest of 8/4/2 CTAs for which the device can hold all rows'
   // clusters at once (a CTA fills an SM, and a cluster has to find its SMs within one GPC).  Rows with explicit
   // ids, and short rows, are not split.
@@ -657,8 +673,9 @@ int launch_topk(const TopkParams& p, int rows, cudaStream_t stream) {
         pattr.val.clusterDim.z = 1;
         probe.attrs = &pattr;
         probe.numAttrs = 1;
+        cudaFuncSetAttribute(topk_select_kernel<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopkClusterSmemBytes);
         int clusters = 0;
-        const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, topk_select_kernel, &probe);
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, topk_select_kernel<false, 1>, &probe);
         if (e != cudaSuccess) cudaGetLastError();
         room[c] = (e == cudaSuccess && clusters > 0) ? clusters : -1;
       }
@@ -670,9 +687,19 @@ int launch_topk(const TopkParams& p, int rows, cudaStream_t stream) {
   // Started while the scores' kernel drains, CTAs of the plain launch pile up two to an SM where that kernel is done first, and
   // scan at half the speed; with few rows there is room and only the latency counts.
   const bool early = csize > 1 || rows <= sm_count() / 4;
-  const int small = p.ids == nullptr && longest <= kSmallRow ? 1 : 0;
+  const bool small = p.ids == nullptr && longest <= kSmallRow;
+  // Two CTAs an SM where rows are more than SMs and what those rows hold stays in L2 from the first scan to the second; rows with
+  // explicit ids are read six times, mostly from memory in either case.  us of a launch with one / two an SM:
+  //   148 rows of 16384, ids: 39 / 49   149 rows: 70 / 51   512 rows: 154 / 108   4096 rows of 131072, ids: 10940 / 6080
+  //   4096 rows of 2048: 180 / 134   of 16384: 408 / 320   of 65536: 627 / 488   scores and top-k of 98304: 4986 / 4966
+  //   beyond L2   scores and top-k of 512 rows of 131072: 848 / 865   4096 rows: 6572 / 6626
+  const bool two = csize == 1 && rows > sm_count() &&
+                   (p.ids != nullptr || 2ll * sm_count() * longest * static_cast<long long>(sizeof(float)) <= l2_bytes());
   const size_t smem = csize > 1 ? kTopkClusterSmemBytes : (small ? kTopkSmallSmemBytes : kTopkSmemBytes);
-  launch_ex(topk_select_kernel, dim3(rows * csize), kTopkThreads, smem, stream, early, csize, p, csize, small);
+  auto kernel = small ? (two ? topk_select_kernel<true, 2> : topk_select_kernel<true, 1>)
+                      : (two ? topk_select_kernel<false, 2> : topk_select_kernel<false, 1>);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTopkClusterSmemBytes);   // (the largest of all)
+  launch_ex(kernel, dim3(rows * csize), kTopkThreads, smem, stream, early, csize, p, csize);
   count_launch();
   return check_launch("topk_select_kernel");
 }

@@ -95,6 +95,30 @@ def test_topk_short_rows(n, k):
     parity.test_topk_exact_order_across_score_distributions(n, k)
 
 
+# one CTA an SM up to 148 rows and two beyond, for rows ordered whole, selected from, and with explicit ids; empty rows among them
+@pytest.mark.parametrize("rows", [148, 149])
+@pytest.mark.parametrize("ld", [2100, 8200])
+@pytest.mark.parametrize("with_ids", [False, True])
+def test_topk_row_counts(rows, ld, with_ids):
+    g = torch.Generator().manual_seed(rows + ld)
+    scores = torch.randn((rows, ld), generator=g).bfloat16().float()   # (ties)
+    counts = torch.randint(0, ld + 1, (rows,), generator=g, dtype=torch.int32)
+    counts[:3] = torch.tensor([0, 1, ld])
+    ids = torch.stack([torch.randperm(2 * ld, generator=g)[:ld] for _ in range(rows)]).int() if with_ids else None
+    if with_ids:
+        ids[:, ::7] = -1   # entries to skip
+    idx, sc = parity._run_topk(scores, counts, 2048, ids=ids)
+    for r in range(rows):
+        n = int(counts[r])
+        v, i = scores[r, :n], ids[r, :n] if with_ids else torch.arange(n, dtype=torch.int32)
+        v, i = v[i >= 0], i[i >= 0]
+        i, order = i.sort()
+        best = v[order].sort(descending=True, stable=True)
+        k = min(2048, i.numel())
+        assert torch.equal(idx[r, :k], i[best.indices[:k]]) and torch.equal(sc[r, :k], best.values[:k]), r
+        assert bool((idx[r, k:] == -1).all()), r
+
+
 # decode batches share their key blocks among the CTAs: lengths alike and ragged, empty requests, more than 128 requests
 @pytest.mark.parametrize("act_seq,s1", [([700] * 5, 2), ([0, 129, 9000, 1, 128, 3000], 1), ([2 + 97 * (i % 40) for i in range(150)], 2)])
 def test_indexer_shares(act_seq, s1):
