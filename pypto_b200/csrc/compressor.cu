@@ -14,8 +14,11 @@
 // state rows a closing window reads were written by the same CTA; only the RMSNorm sum -- and, for the hadamard product, the
 // row -- crosses, through distributed shared memory.  A window that closes with ratio 128 reads 512 KB of state: one CTA took
 // 53 us for it, eight take 10.  Tokens of a request are handled in order because a later token's window contains the rows of
-// the earlier ones.  The kernel adds the projection's partial sums itself and is launched dependent on it.  (The operator for
-// one request of two tokens was two GEMM calls, two reduce kernels, a fill and, rotated, a third GEMM: 115 us of host work.)
+// the earlier ones; between two windows that close nothing is read, and a token's partial sums are fetched under the one before
+// it (1024 tokens of one request, d = 128, hadamard: 2253 us with a fetch, a barrier and look-ups per token and a hadamard product
+// per window, 1326 now, 1452 as separate launches; d = 512: 1622 and 1272).  The kernel adds the projection's partial sums itself
+// and is launched dependent on it.  (The operator for one request of two tokens was two GEMM calls, two reduce kernels, a fill
+// and, rotated, a third GEMM: 115 us of host work.)
 #include <type_traits>
 
 #include "finish.cuh"
@@ -32,19 +35,20 @@ constexpr int kCompMaxD = 512;
 
 // V: columns per thread in the walk over 128 rows (the state rows' alignment allows 16-byte loads if d is a multiple of 4)
 template <int V>
-__global__ void __launch_bounds__(kCompThreads) compressor_update_kernel(CompressorParams p, int csize) {
+__global__ void __launch_bounds__(kCompThreads, 2) compressor_update_kernel(CompressorParams p, int csize) {
   constexpr int kGroups = kCompThreads / (kCompCols / V);   // row groups
   constexpr int kRows = kCompPage / kGroups;                // rows of a thread
   __shared__ float merge_s[kGroups][kCompCols][3];          // (maximum, sum, weighted sum) of a row group, per column
   __shared__ float red_s[2];
   __shared__ float sum_x[2][8];                             // every CTA's sum of squares; two, as a peer may be a window ahead
-  __shared__ float row_x[2][kCompMaxD];                     // the whole row, for the hadamard product
+  __shared__ float row_x[kCompMaxD];                        // the whole row, for the hadamard product
   const int rank = blockIdx.x % csize, b = blockIdx.x / csize, tid = threadIdx.x;
   const int d = p.d, cd = p.coff * p.d, ratio = p.ratio, c0 = rank * kCompCols;
   const int nc = min(kCompCols, d - c0), cc = tid & (kCompCols - 1), grp = tid >> 6;
   pdl_trigger();
   bool closed = false;
   if (b < p.b) {
+    float row_v = 0.f;   // this thread's column of the request's last compressed row
     const int start = p.start_pos[b];
     int nclose = 0;
     pdl_wait();
@@ -53,26 +57,44 @@ __global__ void __launch_bounds__(kCompThreads) compressor_update_kernel(Compres
     const bool score = p.coff == 2 ? (grp >> 1) != 0 : grp != 0;
     const int col = (p.coff == 2 ? (grp & 1) * d : 0) + c0 + cc;
     const bool writes = cc < nc && grp < 2 * p.coff;
-    for (int i = 0; i < p.s1; ++i) {
-      const int pos = start + i;
-      const int lb = pos / kCompPage, cur = pos % kCompPage;
+    const float* sums = (score ? p.score_total : p.kv_total) + static_cast<size_t>(b) * p.s1 * p.ld + col;
+    const size_t split_step = static_cast<size_t>(p.b) * p.s1 * p.ld;
+    float part[16];   // a token's partial sums (a projection is cut into at most 16 splits), fetched a token ahead
+    auto fetch = [&](int i) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        part[k] = writes && i < p.s1 && k < p.splits ? sums[static_cast<size_t>(i) * p.ld + k * split_step] : 0.f;
+    };
+    fetch(0);
+    // The tokens up to the one that closes a window are taken together: they lie in one page, and nothing is read before the last
+    // of them.
+    for (int i = 0, n; i < p.s1; i += n) {
+      const int pos0 = start + i;
+      const int lb = pos0 / kCompPage;
       if (start < 0 || lb >= p.kv_cols || lb >= p.score_cols) {
-        if (tid == 0 && rank == 0) report_status(p.status, DSV32_STATUS_BAD_INDEX, b, pos);
+        if (tid == 0 && rank == 0) report_status(p.status, DSV32_STATUS_BAD_INDEX, b, pos0);
         break;
       }
       const long long kb = p.kv_table[static_cast<size_t>(b) * p.kv_cols + lb];
       const long long sb = p.score_table[static_cast<size_t>(b) * p.score_cols + lb];
       if (kb < 0 || kb >= p.kv_blocks || sb < 0 || sb >= p.score_blocks) {
-        if (tid == 0 && rank == 0) report_status(p.status, DSV32_STATUS_BAD_PAGE, b, pos);
+        if (tid == 0 && rank == 0) report_status(p.status, DSV32_STATUS_BAD_PAGE, b, pos0);
         break;
       }
+      n = min(p.s1 - i, ratio - pos0 % ratio);
       if (writes) {
-        const ProjSums src{score ? p.score_total : p.kv_total, p.b * p.s1, p.ld, p.splits};
-        const float v = proj_sum(src, b * p.s1 + i, col);
-        if (score) p.score_state[(sb * kCompPage + cur) * cd + col] = v + p.ape[static_cast<size_t>(pos % ratio) * cd + col];
-        else p.kv_state[(kb * kCompPage + cur) * cd + col] = v;
+        float* state = (score ? p.score_state + sb * kCompPage * cd : p.kv_state + kb * kCompPage * cd) + col;
+        for (int q = 0; q < n; ++q) {
+          float v = 0.f;
+#pragma unroll
+          for (int k = 0; k < 16; ++k) v += part[k];   // in split order
+          fetch(i + q + 1);
+          const int at = pos0 + q;
+          state[(at % kCompPage) * cd] = score ? v + p.ape[static_cast<size_t>(at % ratio) * cd + col] : v;
+        }
       }
       __syncthreads();  // the rows just written are read below by other threads of this CTA
+      const int pos = pos0 + n - 1;
       if ((pos + 1) % ratio != 0) continue;
 
       // ---- per column: softmax over the rows, weighted sum --------------------------------------------------------
@@ -187,29 +209,30 @@ __global__ void __launch_bounds__(kCompThreads) compressor_update_kernel(Compres
           v = __fadd_rn(__fmul_rn(v, cs), __fmul_rn((j & 1) ? other : -other, sn));
         }
       }
-      __nv_bfloat16* orow = p.out + static_cast<size_t>(b) * d + c0;
-      if (p.hadamard == nullptr) {
-        if (tid < nc) orow[tid] = __float2bfloat16_rn(v);
-      } else {
-        // row x hadamard: every CTA gets the whole row and makes its 64 columns, the reduction over four groups of threads
-        if (tid < nc)
-          for (int r = 0; r < csize; ++r) st_peer_f32(peer_addr(&row_x[par][c0 + tid], r), bf16r(v));
-        if (csize > 1) cluster_arrive_wait();
-        else __syncthreads();
-        float acc = 0.f;
-        if (cc < nc) {
-#pragma unroll 16
-          for (int k = grp; k < d; k += 4)
-            acc = fmaf(row_x[par][k], __bfloat162float(p.hadamard[static_cast<size_t>(k) * d + c0 + cc]), acc);
-        }
-        merge_s[grp][cc][0] = acc;
-        __syncthreads();
-        if (tid < nc)
-          orow[tid] = __float2bfloat16_rn((merge_s[0][tid][0] + merge_s[1][tid][0]) + (merge_s[2][tid][0] + merge_s[3][tid][0]));
-      }
+      if (p.hadamard != nullptr) row_v = bf16r(v);
+      else if (tid < nc) p.out[static_cast<size_t>(b) * d + c0 + tid] = __float2bfloat16_rn(v);
       closed = true;
       ++nclose;
       __syncthreads();  // merge_s / red_s are reused by the next window
+    }
+    if (p.hadamard != nullptr && closed) {   // (alike in all CTAs of the cluster)
+      // Row x hadamard, of the row that stays: a request's later windows overwrite the row of its earlier ones.  Every CTA gets the
+      // whole row and makes its 64 columns, the reduction over four groups of threads.
+      if (tid < nc)
+        for (int r = 0; r < csize; ++r) st_peer_f32(peer_addr(&row_x[c0 + tid], r), row_v);
+      if (csize > 1) cluster_arrive_wait();
+      else __syncthreads();
+      float acc = 0.f;
+      if (cc < nc) {
+#pragma unroll 16
+        for (int k = grp; k < d; k += 4)
+          acc = fmaf(row_x[k], __bfloat162float(p.hadamard[static_cast<size_t>(k) * d + c0 + cc]), acc);
+      }
+      merge_s[grp][cc][0] = acc;
+      __syncthreads();
+      if (tid < nc)
+        p.out[static_cast<size_t>(b) * d + c0 + tid] =
+            __float2bfloat16_rn((merge_s[0][tid][0] + merge_s[1][tid][0]) + (merge_s[2][tid][0] + merge_s[3][tid][0]));
     }
   } else {
     pdl_wait();

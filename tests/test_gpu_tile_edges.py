@@ -74,6 +74,12 @@ def test_compressor_clusters(ratio, rotate, d, starts, s1):
     parity.test_compressor_seeded_vs_oracle(ratio, rotate, d, starts, s1)
 
 
+# many windows of one request in a call: a row that is written over, across pages, from and to the middle of a window
+@pytest.mark.parametrize("ratio,rotate,d,starts,s1", [(4, True, 128, [0, 3, 126], 41), (4, False, 200, [2], 130), (128, True, 128, [0, 77], 300)])
+def test_compressor_windows(ratio, rotate, d, starts, s1):
+    parity.test_compressor_seeded_vs_oracle(ratio, rotate, d, starts, s1)
+
+
 # lists split over idle SMs (few tokens) and not; more items than CTAs; idle lanes; lists shorter than a tile and than a split
 @pytest.mark.parametrize("ori_seq,s1_list,nq,kw", [
     ([4000], [1], 64, {}), ([300, 20], [1, 2], 24, {"topk": 40}), ([2000] * 9, [4] * 9, 64, {"topk": 100}), ([60, 1], [2, 1], 128, {"topk": 8})])
