@@ -59,37 +59,24 @@ __device__ __forceinline__ float hif8_to_float(uint32_t code) {
   }
   return sign * pg_pow2(ev) * (1.f + static_cast<float>(mant) * pg_pow2(-bits));
 }
-__device__ __forceinline__ int hif8_mantissa_bits(int e) {
-  const int ae = e < 0 ? -e : e;
-  return ae <= 3 ? 3 : (ae <= 7 ? 2 : 1);
-}
-// Nearest representable value, a tie to the larger magnitude, magnitudes above 2^15 to 2^15; NaN to the NaN code.
+// Nearest representable value, a tie to the larger magnitude, magnitudes above 2^15 to 2^15; NaN to the NaN code.  Without a
+// branch: the lanes of a warp meet all exponent ranges, and the code of a branch each is long.
 __device__ __forceinline__ uint32_t float_to_hif8(float x) {
-  if (x != x) return 0x80u;
-  const uint32_t sign = (__float_as_uint(x) >> 24) & 0x80u;
-  const float mag = fminf(fabsf(x), 32768.f);
-  if (mag < pg_pow2(-23)) return 0u;                             // nearer to zero, which has no sign
-  int e = static_cast<int>((__float_as_uint(mag) >> 23) & 0xffu) - 127;   // floor(log2(mag)); mag is a normal fp32
-  uint32_t mant = 0u;
-  if (e < -15) {
-    // only powers of two down here: 2^-22 .. 2^-16, then 2^-15 above and zero below; the midpoint goes up
-    if (e == -23 || mag >= 1.5f * pg_pow2(e)) ++e;
-    if (e <= -16) return sign | static_cast<uint32_t>(e + 23);
-  } else {
-    const int bits = hif8_mantissa_bits(e);
-    const float q = mag * pg_pow2(bits - e);                     // in [2^bits, 2^(bits+1)), exact
-    int qi = static_cast<int>(q);                                // floor
-    if (q - static_cast<float>(qi) >= 0.5f) ++qi;                // half away from zero (q - floor(q) is exact)
-    if (qi == (2 << bits)) ++e;                                  // carried into the next exponent, mantissa 0
-    else mant = (static_cast<uint32_t>(qi) & ((1u << bits) - 1u));
-  }
-  const int ae = e < 0 ? -e : e;
-  const uint32_t es = e < 0 ? 1u : 0u;
-  if (ae == 0) return sign | 0x08u | mant;
-  if (ae == 1) return sign | 0x10u | (es << 3) | mant;
-  if (ae <= 3) return sign | 0x20u | (es << 4) | (static_cast<uint32_t>(ae - 2) << 3) | mant;
-  if (ae <= 7) return sign | 0x40u | (es << 4) | (static_cast<uint32_t>(ae - 4) << 2) | mant;
-  return sign | 0x60u | (es << 4) | (static_cast<uint32_t>(ae - 8) << 1) | mant;
+  const uint32_t u = __float_as_uint(x), mag = min(u & 0x7fffffffu, 0x47000000u);   // 2^15
+  const int ae = abs(static_cast<int>(mag >> 23) - 127);
+  const int bits = ae <= 3 ? 3 : (ae <= 7 ? 2 : (ae <= 15 ? 1 : 0));   // mantissa bits at this exponent
+  // half a step is added and the rest cut off; a carry runs into the exponent and leaves no mantissa.  Below 2^-15 there are
+  // only powers of two down to 2^-22, which takes everything from 2^-23 on; what is below is nearer to zero, which has no sign
+  const uint32_t r = mag + (0x400000u >> bits);
+  const int e = max(static_cast<int>(r >> 23) - 127, -22), a = abs(e);
+  const uint32_t m = (r >> (23 - bits)) & ((1u << bits) - 1u), es = e < 0 ? 1u : 0u;
+  const int k = 31 - __clz(a | 1);                                     // prefix of the exponent's width
+  uint32_t code = (static_cast<uint32_t>(k) << 5) | (es << 4) | (static_cast<uint32_t>(a - (1 << k)) << (4 - k));
+  code = a <= 1 ? (a == 0 ? 0x08u : 0x10u | (es << 3)) : code;
+  code = e <= -16 ? static_cast<uint32_t>(e + 23) : code | m;
+  code |= (u >> 24) & 0x80u;
+  code = mag < 0x34000000u ? 0u : code;                                // 2^-23
+  return (u & 0x7fffffffu) > 0x7f800000u ? 0x80u : code;
 }
 
 __device__ __forceinline__ float e8m0_to_float(uint32_t code) {  // 2^(code - 127); code 255 is NaN
@@ -470,52 +457,84 @@ pg_heads_kernel(const __grid_constant__ CUtensorMap a_map, const __grid_constant
       const int b = i & 1;
       if (!__all_sync(0xffffffffu, mbar_wait(&d2full_bar[b], (i >> 1) & 1, p.status, 97))) break;
       tc_fence_after();
-      uint32_t r[2][32];
-      float amax = 0.f;
-      if (warp_live) {
-        tmem_ld_32x32b_x32(lane_base + kPhColD2 + b * 128 + half * 64, r[0]);
-        tmem_ld_32x32b_x32(lane_base + kPhColD2 + b * 128 + half * 64 + 32, r[1]);
-        tmem_ld_wait();
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&d2empty_bar[b]);
-      if (warp_live) {
-#pragma unroll
-        for (int e = 0; e < 64; ++e) {
-          const float v = pg_bf16r(__uint_as_float(r[e >> 5][e & 31]));
-          r[e >> 5][e & 31] = __float_as_uint(v);
-          amax = fmaxf(amax, fabsf(v));
-        }
-      }
+      const uint32_t d2 = lane_base + kPhColD2 + b * 128 + half * 64;
+      uint8_t* dst = p.q_out + (static_cast<size_t>(tk) * p.heads + head) * kPgDim + half * 64;
       float* slot = red + (((i & 1) * 4 + quarter) * 2) * 32;
-      slot[half * 32 + lane] = amax;
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
-      const float scale = pg_row_scale<kMx>(fmaxf(amax, slot[(half ^ 1) * 32 + lane]));
-      if (live) {
-        uint8_t* dst = p.q_out + (static_cast<size_t>(tok) * p.heads + head) * kPgDim + half * 64;
+      auto row_scale = [&](float amax) {   // of both halves
+        slot[half * 32 + lane] = amax;
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
+        return pg_row_scale<kMx>(fmaxf(amax, slot[(half ^ 1) * 32 + lane]));
+      };
+      auto release = [&] {   // D2 has been read
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&d2empty_bar[b]);
+      };
+      auto store16 = [&](int u, const uint32_t* r, float scale) {   // columns 16 u .. of this half
+        uint32_t o[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          uint32_t o[4];
+        for (int e = 0; e < 16; ++e) o[e >> 2] |= pg_code<kMx>(__uint_as_float(r[e]), scale) << (8 * (e & 3));
+        if (vec_out) {
+          reinterpret_cast<uint4*>(dst)[u] = make_uint4(o[0], o[1], o[2], o[3]);
+        } else {
 #pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            uint32_t w = 0;
+          for (int x = 0; x < 4; ++x) store_bytes4(reinterpret_cast<int8_t*>(dst + u * 16 + x * 4), o[x]);
+        }
+      };
+      float scale, amax = 0.f;
+      if constexpr (kMx) {
+        uint32_t r[64];
+        if (warp_live) {
+          tmem_ld_32x32b_x32(d2, *reinterpret_cast<uint32_t(*)[32]>(r));
+          tmem_ld_32x32b_x32(d2 + 32, *reinterpret_cast<uint32_t(*)[32]>(r + 32));
+          tmem_ld_wait();
+        }
+        release();
+        if (warp_live) {
 #pragma unroll
-            for (int y = 0; y < 4; ++y) {
-              const int e = u * 16 + x * 4 + y;
-              w |= pg_code<kMx>(__uint_as_float(r[e >> 5][e & 31]), scale) << (8 * y);
-            }
-            o[x] = w;
-          }
-          if (vec_out) {
-            reinterpret_cast<uint4*>(dst)[u] = make_uint4(o[0], o[1], o[2], o[3]);
-          } else {
-#pragma unroll
-            for (int x = 0; x < 4; ++x) store_bytes4(reinterpret_cast<int8_t*>(dst + u * 16 + x * 4), o[x]);
+          for (int e = 0; e < 64; ++e) {
+            const float v = pg_bf16r(__uint_as_float(r[e]));
+            r[e] = __float_as_uint(v);
+            amax = fmaxf(amax, fabsf(v));
           }
         }
-        if (half == 0) p.q_scale_out[static_cast<size_t>(tok) * p.heads + head] = scale;
+        scale = row_scale(amax);
+        if (live) {
+#pragma unroll
+          for (int u = 0; u < 4; ++u) store16(u, r + 16 * u, scale);
+        }
+      } else {
+        // The columns are read twice, for the maximum and then sixteen at a time in a loop that stays one: the code of 64 of these
+        // conversions in a row is fetched anew by every call (45 KB without a branch in them, 100 with: 27, 44 and 59 us a call at
+        // one token).  For the other format, whose conversion is one instruction, the second reading costs 1.5 us of 33 at 1024.
+        uint32_t r[32];
+        if (warp_live) {
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            tmem_ld_32x32b_x32(d2 + g * 32, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 32; ++e) amax = fmaxf(amax, fabsf(pg_bf16r(__uint_as_float(r[e]))));
+          }
+        }
+        scale = row_scale(amax);
+        if (warp_live) {
+#pragma unroll 1
+          for (int u = 0; u < 4; ++u) {
+            uint32_t q[16];
+            tmem_ld_32x32b_x16(d2 + u * 16, q);
+            tmem_ld_wait();
+            if (live) {   // (rows past the last token hold zeros: zero by zero would take the division's slow path)
+#pragma unroll
+              for (int e = 0; e < 16; ++e) q[e] = __float_as_uint(pg_bf16r(__uint_as_float(q[e])));
+              store16(u, q, scale);
+            }
+            __syncwarp();   // the whole warp loads
+          }
+        }
+        release();
       }
+      if (live && half == 0) p.q_scale_out[static_cast<size_t>(tok) * p.heads + head] = scale;
     }
   }
   tc_fence_before();
