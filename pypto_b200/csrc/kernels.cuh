@@ -82,7 +82,8 @@ struct SfaParams {
 int launch_sfa_tc(const SfaParams& p, cudaStream_t stream);
 int launch_sfa_combine(const SfaParams& p, cudaStream_t stream);
 int launch_scfa_tc(const SfaParams& p, cudaStream_t stream);   // the DeepSeek-V4 form (scfa_tc.cu)
-int scfa_splits(int t, int pair, int slots);
+int scfa_lists(int t, int b, int pair);
+int scfa_splits(int lists, int slots);
 
 struct PrologParams {
   const __nv_bfloat16* x;

@@ -710,10 +710,16 @@ scfa_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
 }
 
 // ---- host ------------------------------------------------------------------------------------------------------------
+// Lists that share the CTAs: one per two tokens where every request has an even number of them and all are paired; otherwise one per
+// token, since the item of a second token, which has nothing to do, takes its turn like the others.
+int scfa_lists(int t, int b, int pair) { return pair && t % b == 0 && t / b % 2 == 0 ? t / 2 : t; }
+
 // Parts a key list is split into: while the items leave SMs idle, and no part below two tiles (a part costs its own Q, O and
-// a share of the combine kernel).
-int scfa_splits(int t, int pair, int slots) {
-  const int lists = pair ? (t + 1) / 2 : t, tiles = (slots + kScTile - 1) / kScTile;
+// a share of the combine kernel).  More items than CTAs would be a second round: 74 requests of one token, once counted as 37 pairs
+// and split in two, took 63.6 us with selected keys and 40.4 with ratio 128, unsplit 33.5 and 16.4; 20 requests of three tokens
+// 47.1 and 30.9, unsplit 32.8 and 16.5.
+int scfa_splits(int lists, int slots) {
+  const int tiles = (slots + kScTile - 1) / kScTile;
   int s = sm_count() / (2 * (lists > 0 ? lists : 1));
   s = s < tiles / 2 ? s : tiles / 2;
   return s < 1 ? 1 : (s > 8 ? 8 : s);
@@ -750,9 +756,9 @@ int launch_scfa_tc(const SfaParams& p, cudaStream_t stream) {
   rc = check_launch("scfa row list kernel");
   if (rc != DSV32_OK) return rc;
   cudaFuncSetAttribute(scfa_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kScSmemBytes));
-  // Persistent CTAs step over (token, half) with a stride of an odd number of tokens: with an even one, CTAs would see first
-  // tokens of pairs only, or none.
-  const int items = 2 * t * p.splits, most = 2 * ((sm_count() / 2 - 1) | 1);
+  // Persistent CTAs step over (token, half) with a stride of an odd number of tokens where there are pairs: with an even one, CTAs
+  // would see first tokens of pairs only, or none.
+  const int items = 2 * t * p.splits, tokens = sm_count() / 2, most = 2 * (p.pair && t != p.b ? (tokens - 1) | 1 : tokens);
   launch_ex(scfa_tc_kernel, dim3(items < most ? items : most), kScThreads, kScSmemBytes, stream, true, 1, q, kv, kv2, run, run2, p, items);
   count_launch();
   rc = check_launch("scfa_tc_kernel");

@@ -80,9 +80,12 @@ def test_compressor_windows(ratio, rotate, d, starts, s1):
     parity.test_compressor_seeded_vs_oracle(ratio, rotate, d, starts, s1)
 
 
-# lists split over idle SMs (few tokens) and not; more items than CTAs; idle lanes; lists shorter than a tile and than a split
+# lists split over idle SMs (few tokens) and not; more items than CTAs; idle lanes; lists shorter than a tile and than a split;
+# no pairs, pairs beside single tokens, requests of different numbers of tokens
 @pytest.mark.parametrize("ori_seq,s1_list,nq,kw", [
-    ([4000], [1], 64, {}), ([300, 20], [1, 2], 24, {"topk": 40}), ([2000] * 9, [4] * 9, 64, {"topk": 100}), ([60, 1], [2, 1], 128, {"topk": 8})])
+    ([4000], [1], 64, {}), ([300, 20], [1, 2], 24, {"topk": 40}), ([700] * 37, [1] * 37, 64, {"topk": 100}),
+    ([200] * 74, [1] * 74, 16, {"topk": 60}), ([900] * 12, [3] * 12, 64, {"topk": 100}), ([400] * 7, [1, 2, 3, 4, 5, 6, 7], 32, {"topk": 60}),
+    ([2000] * 9, [4] * 9, 64, {"topk": 100}), ([60, 1], [2, 1], 128, {"topk": 8})])
 def test_compressed_attention_splits(ori_seq, s1_list, nq, kw):
     d = helpers.gen_scfa_inputs(900 + len(ori_seq) + nq, ori_seq, s1_list, nq=nq, **kw)
     # (with few keys the rounding of the probabilities shows in more last bits)
