@@ -245,13 +245,23 @@ class Dsv32Error(RuntimeError):
 
 
 def _import_front():
-    import torch  # noqa: F401  (its libraries come first: the front end links against them)
     importlib.invalidate_caches()   # the file may have been built by this very process
     try:
         return importlib.import_module("._front", __package__)
     except ImportError as e:
         raise Dsv32Error(f"the native front end (_front.so) cannot be imported: {e}; "
                          "build it with `python -m pypto_b200.build`") from e
+
+
+def _load_front():
+    """The front end, if it was compiled for this binding's argument blocks and for the torch that is loaded."""
+    import torch   # (its libraries come first: the front end links against them)
+    native = _import_front()
+    for what, has, wants in (("ABI", native.ABI_VERSION, ABI_VERSION), ("torch", native.TORCH_VERSION, torch.__version__.split("+")[0])):
+        if has != wants:
+            raise Dsv32Error(f"the native front end (_front.so) was built for {what} {has}, this is {what} {wants}: "
+                             "build it again with `python -m pypto_b200.build --force`")
+    return native
 
 
 def load():
@@ -269,7 +279,7 @@ def load():
         fn.argtypes = args
     if lib.dsv32_abi_version() != ABI_VERSION:
         raise Dsv32Error(f"ABI mismatch: library {lib.dsv32_abi_version()}, binding {ABI_VERSION}")
-    native = _import_front()
+    native = _load_front()
     native.bind({name: C.cast(getattr(lib, name), c_void_p).value for name in EXPORTS}, check)
     _lib, front = lib, native
     for index, address in list(_status_words.items()):

@@ -20,6 +20,7 @@ LIB_PATH = os.path.join(HERE, LIB_NAME)
 SOURCES = ["api.cu", "topk.cu", "indexer_tc.cu", "sfa_tc.cu", "scfa_tc.cu", "sfa_combine.cu", "gemm_tc.cu", "heads_tc.cu", "prolog_finish.cu", "prolog_v4.cu", "v4_q_tc.cu", "pg_prolog.cu",
            "mla_prolog_v4.cu", "hc_pre.cu", "hc_pre_tc.cu", "compressor.cu", "decode_advance.cu", "noalloc.cu"]
 FRONT_SOURCE, FRONT_PATH = os.path.join(CSRC, "front.cpp"), os.path.join(HERE, "_front.so")
+FRONT_TORCH = os.path.join(HERE, "build", "front_torch")   # the torch release _front.so was linked against
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -44,7 +45,16 @@ def _newest_source_mtime() -> float:
 
 def is_stale() -> bool:
     newest = _newest_source_mtime()
-    return any(not os.path.exists(p) or os.path.getmtime(p) < newest for p in (LIB_PATH, FRONT_PATH))
+    return any(not os.path.exists(p) or os.path.getmtime(p) < newest for p in (LIB_PATH, FRONT_PATH)) or not _front_fits_torch()
+
+
+def _front_fits_torch() -> bool:
+    import torch
+    try:
+        with open(FRONT_TORCH) as f:
+            return f.read() == torch.__version__
+    except OSError:
+        return False
 
 
 def _front_command() -> list:
@@ -83,7 +93,10 @@ def build(verbose: bool = False, force: bool = False) -> str:
             sys.stderr.write(f"--- {os.path.basename(src)} ---\n{out}\n")
         failed |= pr.returncode != 0
     if failed:
-        raise RuntimeError("nvcc failed; see output above")
+        raise RuntimeError("nvcc or g++ failed; see output above")
+    import torch
+    with open(FRONT_TORCH, "w") as f:
+        f.write(torch.__version__)
     link = [nvcc_path(), *ARCH_FLAGS, "-shared", "-o", LIB_PATH, *objs, "-lcudart"]
     res = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if res.returncode != 0:

@@ -20,6 +20,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/version.h>
 
 #include <algorithm>
 #include <cstring>
@@ -782,4 +783,13 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_front", "Native front end of the 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__front(void) { return PyModule_Create(&module); }
+// What this file was compiled for: its argument blocks follow the header of that version, its calls torch's of that release.
+PyMODINIT_FUNC PyInit__front(void) {
+  PyObject* m = PyModule_Create(&module);
+  if (m == nullptr || PyModule_AddIntConstant(m, "ABI_VERSION", DSV32_ABI_VERSION) != 0 ||
+      PyModule_AddStringConstant(m, "TORCH_VERSION", TORCH_VERSION) != 0) {
+    Py_XDECREF(m);
+    return nullptr;
+  }
+  return m;
+}

@@ -5,6 +5,7 @@ import subprocess
 import sys
 
 import pytest
+import torch
 
 import helpers
 from pypto_b200 import _lib
@@ -71,13 +72,46 @@ def test_missing_front_end_is_an_error_that_says_so(checkout, built):
     assert "circular import" not in r.stderr
 
 
+class _Front:
+    """Stands in for the native module."""
+    ABI_VERSION, TORCH_VERSION = _lib.ABI_VERSION, torch.__version__.split("+")[0]
+
+    def bind(self, *args):
+        pass
+
+    def set_status(self, *args):
+        pass
+
+
+@pytest.mark.parametrize("name,value", [("ABI_VERSION", _lib.ABI_VERSION - 1), ("TORCH_VERSION", "1.0.0")])
+def test_front_end_of_another_build_is_refused(built, monkeypatch, name, value):
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib, "_import_front", type("Front", (_Front,), {name: value}))
+    with pytest.raises(_lib.Dsv32Error, match=f"built for .* {value}"):
+        _lib.load()
+
+
+def test_front_end_says_what_it_was_built_for(built):
+    _lib.load()
+    assert (_lib.front.ABI_VERSION, _lib.front.TORCH_VERSION) == (_Front.ABI_VERSION, _Front.TORCH_VERSION)
+
+
+def test_front_end_linked_against_another_torch_is_stale(built, monkeypatch, tmp_path):
+    from pypto_b200 import build
+    stamp = tmp_path / "front_torch"
+    monkeypatch.setattr(build, "FRONT_TORCH", str(stamp))
+    monkeypatch.setattr(build, "_newest_source_mtime", lambda: 0.0)
+    assert build.is_stale()
+    stamp.write_text("1.0.0")
+    assert build.is_stale()
+    stamp.write_text(torch.__version__)
+    assert not build.is_stale()
+
+
 def test_status_words_made_before_the_load_reach_the_front_end(built, monkeypatch):
     seen = []
 
-    class Front:
-        def bind(self, *args):
-            pass
-
+    class Front(_Front):
         def set_status(self, *args):
             seen.append(args)
 
