@@ -19,7 +19,7 @@
 extern "C" {
 #endif
 
-#define DSV32_ABI_VERSION 2
+#define DSV32_ABI_VERSION 3   /* 3: Dsv32HcPreArgs has a status word */
 
 /* host-side return codes */
 #define DSV32_OK 0
@@ -564,6 +564,7 @@ typedef struct {
   float* comb;                    /* out fp32 [t, 4, 4]                   */
   void* workspace;                /* >= dsv32_hc_pre_workspace_bytes(t), 16-byte aligned */
   size_t workspace_bytes;
+  uint32_t* status;               /* device uint32[4] or NULL             */
   int32_t t, hc_mult, d, iters;   /* hc_mult must be 4, d 4096, iters >= 1 */
   float norm_eps, hc_eps;
 } Dsv32HcPreArgs;

@@ -101,8 +101,8 @@ class CompressorOpArgs(C.Structure):
 class HcPreArgs(C.Structure):
     _fields_ = [
         ("x", c_void_p), ("hc_fn", c_void_p), ("hc_scale", c_void_p), ("hc_base", c_void_p), ("y", c_void_p),
-        ("post", c_void_p), ("comb", c_void_p), ("workspace", c_void_p), ("workspace_bytes", c_size_t), ("t", c_i32),
-        ("hc_mult", c_i32), ("d", c_i32), ("iters", c_i32),
+        ("post", c_void_p), ("comb", c_void_p), ("workspace", c_void_p), ("workspace_bytes", c_size_t),
+        ("status", c_void_p), ("t", c_i32), ("hc_mult", c_i32), ("d", c_i32), ("iters", c_i32),
         ("norm_eps", c_float), ("hc_eps", c_float),
     ]
 
@@ -236,7 +236,7 @@ EXPORTS = {
     "dsv32_gemm_i8": (c_i32, [C.POINTER(GemmI8Args), c_void_p]),
 }
 
-ABI_VERSION = 2
+ABI_VERSION = 3
 _lib = None
 
 

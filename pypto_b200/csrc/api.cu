@@ -793,6 +793,7 @@ int dsv32_hc_pre(const Dsv32HcPreArgs* a, void* cuda_stream) {
   p.y = static_cast<__nv_bfloat16*>(a->y);
   p.post = a->post;
   p.comb = a->comb;
+  p.status = a->status;
   p.t = a->t;
   p.iters = a->iters;
   p.norm_eps = a->norm_eps;

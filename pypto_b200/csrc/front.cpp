@@ -638,6 +638,7 @@ PyObject* hc_pre(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Scratch ws(p_dsv32_hc_pre_workspace_bytes(g.t));
   g.workspace = ws.ptr();
   g.workspace_bytes = ws.bytes;
+  g.status = g_status[c.dev];
   if (fail(p_dsv32_hc_pre(&g, c.stream()), "hc_pre")) return nullptr;
   if (n == 10) Py_RETURN_TRUE;
   return Py_BuildValue("(NNN)", THPVariable_Wrap(std::move(y)), THPVariable_Wrap(std::move(post)), THPVariable_Wrap(std::move(comb)));

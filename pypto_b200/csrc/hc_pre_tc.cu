@@ -187,7 +187,7 @@ hc_pre_dots_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_co
       if (c >= kHtSeg && c % kHtSeg == kHtDrainLag) drain();
     }
     while (ok && drained < segs) drain();
-    if (!ok) {   // a wait ran out (never seen): there is no status word to report to in this operator's arguments
+    if (!ok) {   // a wait ran out (the status word has it): the sums are not to be taken for results
       sq0 = acc[0] = __int_as_float(0x7fc00000);
 #pragma unroll
       for (int j = 1; j < 16; ++j) acc[j] = acc[0];

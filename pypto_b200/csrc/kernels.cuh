@@ -314,7 +314,7 @@ struct HcPreParams {
   float* post;              // [t, 4]
   float* comb;              // [t, 4, 4]
   float* partial;           // workspace: [groups, t, 24] partial dot products, or with sums of squares [splits, t, kHcPartLd]
-  uint32_t* status;         // may be NULL
+  uint32_t* status;
   int t, iters;
   float norm_eps, hc_eps;
 };

@@ -50,8 +50,8 @@ def hc_pre_kernel(x, hc_fn, hc_scale, hc_base, y, post, comb, hc_mult=4, hc_spli
         ws_bytes = lib.dsv32_hc_pre_workspace_bytes(t)
         ws = rt.workspace(ws_bytes, dev)
         a = _lib.HcPreArgs(rt.ptr(x), rt.ptr(hc_fn), rt.ptr(hc_scale), rt.ptr(hc_base), rt.ptr(y), rt.ptr(post),
-                           rt.ptr(comb), rt.ptr(ws), int(ws_bytes), t, HC_MULT, D, int(hc_split_sinkhorn_iters),
-                           NORM_EPS, float(hc_eps))
+                           rt.ptr(comb), rt.ptr(ws), int(ws_bytes), rt.ptr(rt.status_word(dev)), t, HC_MULT, D,
+                           int(hc_split_sinkhorn_iters), NORM_EPS, float(hc_eps))
         rt.check(lib.dsv32_hc_pre(C.byref(a), rt.stream_ptr(dev)), "hc_pre")
     return None
 

@@ -30,6 +30,30 @@ def test_header_and_binding_agree():
     assert _header_symbols() == sorted(_lib.EXPORTS)
 
 
+def _header_structs():
+    """{name: field names in order} of the argument structs the public header declares."""
+    with open(os.path.join(helpers.ROOT, "include", "dsv32_b200.h")) as f:
+        text = re.sub(r"/\*.*?\*/", "", f.read(), flags=re.S)
+    out = {}
+    for body, name in re.findall(r"typedef struct \{(.*?)\} (Dsv32\w+);", text, flags=re.S):
+        out[name] = [re.search(r"(\w+)\s*(?:\[\w+\])?\s*$", d).group(1) for line in body.split(";") for d in line.split(",") if d.strip()]
+    return out
+
+
+def test_argument_blocks_follow_the_header():
+    structs = _header_structs()
+    assert len(structs) > 15
+    for name, fields in structs.items():
+        assert [f[0] for f in getattr(_lib, name[len("Dsv32"):])._fields_] == fields, name
+
+
+def test_every_operator_that_waits_has_a_status_word():
+    # kernels wait with a limit and report a wait that ran out; these blocks belong to kernels without waits, or hold other blocks
+    no_waits = {"Dsv32TopkArgs", "Dsv32TopkScatter", "Dsv32MlaV4StageArgs", "Dsv32FusedPrologArgs"}
+    for name, fields in _header_structs().items():
+        assert ("status" in fields) != (name in no_waits), name
+
+
 def test_library_exports_every_declared_symbol(lib):
     for name in _header_symbols():
         assert hasattr(lib, name), name
