@@ -560,8 +560,9 @@ static int indexer_prolog_fill(const Dsv32PrologArgs* a, PrologParams& p, bool o
   REQUIRE(reinterpret_cast<uintptr_t>(a->q_norm) % 16 == 0 && reinterpret_cast<uintptr_t>(a->w_qb) % 16 == 0 &&
               reinterpret_cast<uintptr_t>(a->hadamard_q) % 16 == 0 && reinterpret_cast<uintptr_t>(a->hadamard_k) % 16 == 0 &&
               reinterpret_cast<uintptr_t>(a->x) % 16 == 0 && reinterpret_cast<uintptr_t>(a->wk) % 16 == 0 &&
-              reinterpret_cast<uintptr_t>(a->w_proj) % 16 == 0,
-          "prolog: x / q_norm / weights / hadamard matrices must be 16-byte aligned");
+              reinterpret_cast<uintptr_t>(a->w_proj) % 16 == 0 && reinterpret_cast<uintptr_t>(a->q_int8) % 16 == 0 &&
+              reinterpret_cast<uintptr_t>(a->cos_idx_rope) % 4 == 0 && reinterpret_cast<uintptr_t>(a->sin_idx_rope) % 4 == 0,
+          "prolog: x / q_norm / weights / hadamard matrices / q_int8 must be 16-byte aligned, cos / sin 4-byte aligned");
   REQUIRE(a->cache_rows >= 1, "prolog: cache_rows=%lld must be >= 1", static_cast<long long>(a->cache_rows));
   const size_t need = dsv32_prolog_workspace_bytes(a->t);
   if (own_workspace && (a->workspace == nullptr || a->workspace_bytes < need)) {
@@ -742,6 +743,7 @@ int dsv32_mla_prolog_v4(const Dsv32MlaPrologV4Args* a, void* cuda_stream) {
   REQUIRE(((reinterpret_cast<uintptr_t>(a->x) | reinterpret_cast<uintptr_t>(a->wq_a) | reinterpret_cast<uintptr_t>(a->wq_b) |
             reinterpret_cast<uintptr_t>(a->wkv) | reinterpret_cast<uintptr_t>(a->q_out) | reinterpret_cast<uintptr_t>(a->qr)) & 15u) == 0,
           "mla v4: x, the weights, q_out and qr must be 16-byte aligned");
+  REQUIRE(((reinterpret_cast<uintptr_t>(a->cos) | reinterpret_cast<uintptr_t>(a->sin)) & 3u) == 0, "mla v4: cos and sin must be 4-byte aligned");
   const size_t need = mla_v4_workspace_bytes(a->t, a->h);
   if (a->workspace == nullptr || a->workspace_bytes < need) {
     set_error("mla v4: workspace of %zu bytes required, got %zu", need, a->workspace_bytes);

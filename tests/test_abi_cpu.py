@@ -106,6 +106,32 @@ def test_host_side_rejections(lib):
     assert lib.dsv32_indexer_prolog(C.byref(p), None) == -1
 
 
+def _filled(block):
+    """An argument block with aligned pointers, small sizes and no workspace: it is turned down for the workspace, the last check."""
+    for name, kind in block._fields_:
+        if kind is C.c_void_p:
+            setattr(block, name, 0x1000)
+        elif kind is C.c_float:
+            setattr(block, name, 1e-6)
+        else:
+            setattr(block, name, 0 if name == "workspace_bytes" else 2)
+    return block
+
+
+@pytest.mark.parametrize("entry,block,field,to", [
+    ("dsv32_indexer_prolog", _lib.PrologArgs, "q_int8", 16), ("dsv32_indexer_prolog", _lib.PrologArgs, "cos_idx_rope", 4),
+    ("dsv32_indexer_prolog", _lib.PrologArgs, "sin_idx_rope", 4), ("dsv32_mla_prolog_v4", _lib.MlaPrologV4Args, "cos", 4),
+    ("dsv32_mla_prolog_v4", _lib.MlaPrologV4Args, "sin", 4)])
+def test_wide_accesses_are_not_launched_on_unaligned_tensors(lib, entry, block, field, to):
+    a = _filled(block())
+    if block is _lib.MlaPrologV4Args:
+        a.h, a.quant = 64, 1
+    assert getattr(lib, entry)(C.byref(a), None) == -2, lib.dsv32_last_error()
+    setattr(a, field, 0x1000 + to // 2)
+    assert getattr(lib, entry)(C.byref(a), None) == -1
+    assert b"aligned" in lib.dsv32_last_error()
+
+
 def test_python_entry_points_fail_loudly_without_gpu():
     if torch.cuda.is_available():
         pytest.skip("GPU present")
