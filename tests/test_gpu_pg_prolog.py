@@ -61,7 +61,7 @@ def _values(codes_u8, fmt):
     return codes_u8.view(torch.float8_e4m3fn).float() if fmt == "mxfp8" else pgo.hif8_decode(codes_u8)
 
 
-def _check(inp, fmt, got, golden=None):
+def _check(inp, fmt, got, golden=None, weights_rtol=2 ** -7, weights_atol=1e-6):
     q, q_scale, pages_after, weights = got
     t = inp["x"].shape[0]
     heads = inp["w_proj"].shape[1]
@@ -97,7 +97,7 @@ def _check(inp, fmt, got, golden=None):
     assert same_q >= 0.97 and same_k >= 0.97, (same_q, same_k)
     assert torch.allclose(q_scale.reshape(-1), bqs.reshape(-1), rtol=1e-2, atol=0)
     assert torch.allclose(k_scales, bks.reshape(-1), rtol=1e-2, atol=0)
-    assert torch.allclose(weights.float(), bw.float(), rtol=2 ** -7, atol=1e-6)
+    assert torch.allclose(weights.float(), bw.float(), rtol=weights_rtol, atol=weights_atol)
 
 
 def test_pg_prolog_mxfp8_reference_golden_fixture():

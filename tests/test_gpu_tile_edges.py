@@ -139,16 +139,9 @@ def test_indexer_shares(act_seq, s1):
 @pytest.mark.parametrize("t", [128, 129, 257])
 def test_pg_prolog_tiles(fmt, t):
     inp = helpers.gen_pg_prolog_inputs(920 + t, t, fmt)
-    q, q_scale, pages, weights = pg._run(inp, fmt)
-    rq, rqs, rk, rks, rw = pg.pgo.pg_prolog(fmt=fmt, **pg._oracle_args(inp))
-    k_cache, k_scales = helpers.pg_cache_views(pages, fmt)
-    rows = inp["cache_index"].reshape(-1)
-    codes = lambda v: v.reshape(-1).view(torch.uint8)  # noqa: E731
-    assert (codes(q) == codes(rq)).float().mean() >= 0.97
-    assert (codes(k_cache.reshape(-1, 128)[rows]) == codes(rk)).float().mean() >= 0.97
-    assert torch.allclose(q_scale.reshape(-1), rqs.reshape(-1), rtol=1e-2, atol=0)
-    assert torch.allclose(k_scales.reshape(-1)[rows], rks.reshape(-1), rtol=1e-2, atol=0)
-    assert torch.allclose(weights.float(), rw.float(), rtol=2 ** -6, atol=1e-5)   # three roundings to bf16, any of which may flip
+    # a head weight is rounded to bf16 three times; the first rounding may fall the other way (2^-7 of it at most) and take the last
+    # one with it, and a weight near zero keeps the absolute error of its 2560-long sum
+    pg._check(inp, fmt, pg._run(inp, fmt), weights_rtol=2 ** -6, weights_atol=1e-5)
 
 
 def test_pg_prolog_unaligned_weights():

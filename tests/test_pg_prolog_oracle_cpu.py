@@ -4,9 +4,11 @@ accuracy rule, and the HiF8 codec against the facts the reference's decoder stat
 import math
 
 import numpy as np
+import pytest
 import torch
 
 import helpers
+import test_gpu_pg_prolog as on_gpu
 from oracle import pg_prolog_oracle as pgo
 
 
@@ -83,3 +85,27 @@ def test_hif8_operator_restatement_is_self_consistent():
     top = pgo.hif8_decode(q).abs().amax(dim=-1)
     assert torch.all(top == 32768.0)
     assert torch.isfinite(w.float()).all() and ks.shape == (3, 1)
+
+
+@pytest.mark.parametrize("fmt", ["mxfp8", "hif8"])
+@pytest.mark.parametrize("wrong", [None, "q", "k"])
+def test_gpu_comparison_sees_one_wrong_token_past_a_tile(fmt, wrong):
+    # the operator restatement in the place of the GPU's results, as it is and with the codes of token 129 of 129 out of order
+    t = 129
+    inp = helpers.gen_pg_prolog_inputs(920 + t, t, fmt)
+    q, q_scale, k, k_scale, weights = pgo.pg_prolog(fmt=fmt, **on_gpu._oracle_args(inp))
+    q, k = q.view(torch.uint8).reshape(t, -1).clone(), k.view(torch.uint8).reshape(t, 128).clone()
+    if wrong is not None:
+        codes = q if wrong == "q" else k
+        codes[-1] = codes[-1].flip(0)
+    pages = inp["pages"].clone()
+    k_cache, k_scale_cache = helpers.pg_cache_views(pages, fmt)
+    page, slot = (inp["cache_index"].reshape(-1) // helpers.PG_BS, inp["cache_index"].reshape(-1) % helpers.PG_BS)
+    k_cache[page, slot, 0] = k.view(k_cache.dtype)
+    k_scale_cache[page, slot, 0, 0] = k_scale.reshape(-1)
+    got = (q.reshape(-1, 128), q_scale.reshape(-1, 1), pages, weights)
+    if wrong is None:
+        on_gpu._check(inp, fmt, got)
+    else:
+        with pytest.raises(AssertionError, match=f"{wrong}: error ratios"):
+            on_gpu._check(inp, fmt, got)
