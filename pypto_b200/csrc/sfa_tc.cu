@@ -12,8 +12,8 @@
 // stages of 64 gathered keys x 576 dims (nine 64x64 bf16 chunks, 128-byte swizzle).  A stage is read
 // K-major by S = Q K^T and MN-major (as V) by O += P V, so the dequantised rows are written once.
 // Warps: 0 = issuer of the S MMAs / tensor-memory owner, 1..4 = softmax + O rescale + epilogue (one head per
-// thread, so row max / row sum need no shuffles; lane 0 of warp 1 also issues the PV MMAs), 5..20 = gather +
-// dequantise producers (raw rows held in registers two tiles ahead of their use).  A stage is refilled in two steps: the chunks only S reads (the other half's value
+// thread, so row max / row sum need no shuffles; warp 1 also issues the PV MMAs), 5..20 = gather +
+// dequantise producers (raw rows held in registers one tile ahead of their use).  A stage is refilled in two steps: the chunks only S reads (the other half's value
 // dims, the rope dims) as soon as S of the tile two back has completed, this CTA's own value chunks once its
 // PV has.  The cache row of every selected key comes from a pre-pass (sfa_row_ids_kernel).
 // The running maximum is only raised when a tile exceeds it by more than 2^8 (warp-uniform decision), so
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kStThreads, 1) sfa_tc_kernel(const __grid_cons
       tc_fence_before();
       mbar_arrive(&pready_bar[s]);
       if (warp == 1) {  // second MMA issuer: PV of this tile, as soon as all four softmax warps have stored P
-        // (the whole warp waits and computes the uniform operands; lane 0 issues)
+        // (the whole warp waits and computes the uniform operands; one elected lane issues)
         if (!__all_sync(0xffffffffu, mbar_wait(&pready_bar[s], (i >> 1) & 1, p.status, 13))) { ok = false; break; }
         constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 256, false, true);
         constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024, version 1, 128-byte swizzle
@@ -448,19 +448,14 @@ __global__ void __launch_bounds__(kStThreads, 1) sfa_tc_kernel(const __grid_cons
   } else {
     // ================================ gather + dequantise producers ========================================
     // 512 threads: thread (gkey, gpart) owns the 16-byte column gpart of every 128-byte group of key row gkey of
-    // each tile.  Raw rows travel global -> registers TWO tiles ahead of their use (two register sets that
-    // alternate by tile parity; one set for the bf16 caches, whose rows are twice as wide), are dequantised and
-    // stored into the swizzled K stage once the MMAs of the tile two back have released it.
+    // each tile.  Raw rows travel global -> registers one tile ahead of their use, are dequantised and stored into the
+    // swizzled K stage once the MMAs of the tile two back have released it.
     const int ptid = tid - 160;            // 0..511
     const int gkey = ptid >> 3, gpart = ptid & 7;
     const int pw = warp - 5;               // this warp's rows of a tile: 4*pw .. 4*pw + 3
-#ifndef DSV32_SFA_DEPTH
-#define DSV32_SFA_DEPTH 1
-#endif
-    constexpr int kDepth = kBf16 ? 1 : DSV32_SFA_DEPTH;  // register sets = tiles of raw rows in flight
     // The cache row of every selected key was resolved by the pre-pass (row + 1, 0 = none).  Row ids travel
     // global -> shared memory with 4-byte cp.async six tiles ahead (ring of eight tiles per warp), so that the
-    // L2 prefetch (four tiles ahead) and the loads (kDepth tiles ahead) find them in place.
+    // L2 prefetch (four tiles ahead) and the loads (one tile ahead) find them in place.
     int* ring = ring_s + pw * (kStRingTiles * 4);
     const int32_t* ids_row = p.row_ids + static_cast<size_t>(tok) * p.topk;
     auto fetch_ids = [&](int tile) {
@@ -565,7 +560,7 @@ __global__ void __launch_bounds__(kStThreads, 1) sfa_tc_kernel(const __grid_cons
       store_group(stage, q_oth + 1, lo, hi);
       *reinterpret_cast<int4*>(stage + off_rope) = pf.valid ? pf.rope : make_int4(0, 0, 0, 0);
     };
-    // One tile: refill its stage from `pf`, then start the loads of the tile kDepth ahead into the same registers.
+    // One tile: refill its stage from `pf`, then start the loads of the next into the same registers.
     auto do_tile = [&](int i, StPrefetch& pf) -> bool {
       const int s = i & 1;
       // Once S of tile i-2 has completed, every chunk of the stage except this CTA's own value chunks is free
@@ -589,31 +584,27 @@ __global__ void __launch_bounds__(kStThreads, 1) sfa_tc_kernel(const __grid_cons
       fence_proxy_async_smem();  // generic-proxy stores -> visible to the tensor-core (async) proxy
       __syncwarp();
       if (lane == 0) mbar_arrive(&full_bar[s]);
-      // The loads of the tile kDepth ahead go out after the hand-over: issued before the wait above they hold the
+      // The loads of the next tile go out after the hand-over: issued before the wait above they hold the
       // warp at the load/store unit (its miss queue is the scarce resource) and the hand-over comes later (measured).
       fetch_ids(i + 6);
       asm volatile("cp.async.wait_group 2;" ::: "memory");   // ids up to tile i + 4 have landed
       __syncwarp();
-      if (i + kDepth < ntiles) issue_loads(row_of(i + kDepth), pf);
+      if (i + 1 < ntiles) issue_loads(row_of(i + 1), pf);
       if (i + 4 < ntiles) l2_prefetch(row_of(i + 4));
       return true;
     };
 
     pdl_wait();   // the rows are the pre-pass'
-    StPrefetch pfA, pfB;
+    StPrefetch pf;
     for (int tl = 0; tl < 6; ++tl) fetch_ids(tl);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncwarp();
-    issue_loads(row_of(0), pfA);
-    if constexpr (kDepth == 2) {
-      if (1 < ntiles) issue_loads(row_of(1), pfB);
-      else pfB.valid = false;
-    }
-    for (int tl = kDepth; tl < 4; ++tl)
+    issue_loads(row_of(0), pf);
+    for (int tl = 1; tl < 4; ++tl)
       if (tl < ntiles) l2_prefetch(row_of(tl));
-    for (int i = 0; i < ntiles; i += 2) {
-      if (!do_tile(i, pfA)) break;
-      if (i + 1 < ntiles && !do_tile(i + 1, kDepth == 2 ? pfB : pfA)) break;
+    for (int i = 0; i < ntiles; i += 2) {   // (both stages in a turn: fewer spills)
+      if (!do_tile(i, pf)) break;
+      if (i + 1 < ntiles && !do_tile(i + 1, pf)) break;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");   // no row-id copy may still be in flight at exit
   }
