@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(TcShape<TOK>::kThreads, TOK <= 2 ? 2 : 1) inde
   const int ntok = min(TOK, p.s1 - tok0);
   const int bs = 128;
   int b = blockIdx.y, blk_begin, blk_end, hi;
-  if constexpr (TOK > 2) {   // a prefill chunk: always the host's number of blocks
+  if constexpr (TOK > 2) {   // three tokens or more a request: always the host's number of blocks, chosen for the longest request
     blk_begin = p.key_begin / bs + blockIdx.x * p.blocks_per_cta;
     blk_end = min(blk_begin + p.blocks_per_cta, p.key_begin / bs + tc_blocks(p, b, blockIdx.x == 0 && tid == 0, hi));
     if (blk_begin >= blk_end) return;   // uniform for the CTA
@@ -477,8 +477,9 @@ int launch_indexer_scores_tc(const IndexerParams& p, cudaStream_t stream) {
   if (rc != DSV32_OK) return rc;
   IndexerParams q = p;
   if (p.b > 1 && p.s1 <= 2 && p.b < (1 << 20)) {
-    // A decode batch: the CTAs share the blocks among themselves (tc_share).  At most four rounds while no share outgrows a
-    // CTA's page table: more would mostly be CTAs that find nothing to do.
+    // A decode batch of up to two tokens a request: the CTAs share the blocks among themselves (tc_share; not built for TOK = 4,
+    // where a ragged batch still runs the blocks of its longest request).  At most four rounds while no share outgrows a CTA's page
+    // table: more would mostly be CTAs that find nothing to do.
     const long long slots = 2ll * sm_count(), most = static_cast<long long>(nblk) * p.b;
     long long rounds = (most / 56 + p.b / 2 + slots / 2) / slots;
     const long long need = most / (kTcBlocksPerCta - 1) / slots + 1;

@@ -687,6 +687,7 @@ int launch_topk(const TopkParams& p, int rows, cudaStream_t stream) {
   // Started while the scores' kernel drains, CTAs of the plain launch pile up two to an SM where that kernel is done first, and
   // scan at half the speed; with few rows there is room and only the latency counts.
   const bool early = csize > 1 || rows <= sm_count() / 4;
+  // (What the host knows of a row's length is the width of the page table: behind a wider one short rows are selected from.)
   const bool small = p.ids == nullptr && longest <= kSmallRow;
   // Two CTAs an SM where rows are more than SMs and what those rows hold stays in L2 from the first scan to the second; rows with
   // explicit ids are read six times, mostly from memory in either case.  us of a launch with one / two an SM:
