@@ -272,31 +272,27 @@ size_t prolog_partial_bytes(int t, bool mla, bool indexer) {
 // How the indexer prolog on its own runs: its heads take q_norm as an input, so they can run beside projection and finish.  A
 // heads CTA needs an SM to itself (200 KB of shared memory, 53,760 registers), and a finish CTA that was launched early and waits
 // for the projection keeps it from one: with the finish always before the heads the call went from 16.7 to 22.5 us where a CTA
-// per token and 64 heads' CTAs no longer fit the SMs.  Three forms in which nothing waits for an SM:
-//   finish, heads; a CTA per token          while finish and heads CTAs fit
-//   finish, heads; a warp per token         while projection, finish and heads CTAs fit
-//   heads, finish; a CTA per token          while the heads make at most two rounds: they take the CTAs of whole rounds, the
-//                                           projection the SMs they leave, in no more splits than it needs to be done with them
-// us at 64, 128, 192, 256, 384 and 512 tokens, everything read from memory:   16.4  18.5  20.2  20.5  28.0  28.8
-//   the finish always before the heads                                        16.2  24.4  26.7  29.2  30.8  37.1
-//   the heads on a second stream                                              18.6  20.9  22.9  25.9  28.8  36.7
-// Beyond that every kernel fills the chip by itself (1024 tokens: 45 us in the first order, 62 on two streams).
+// per token and 64 heads' CTAs no longer fit the SMs.  Two forms in which nothing waits for an SM:
+//   finish, heads     while finish and heads CTAs fit
+//   heads, finish     while the heads make at most two rounds: they take the CTAs of whole rounds, and the projection the SMs they
+//                     leave, in no more splits than it needs to be done with them
+// us at 64, 128, 192, 256, 384 and 512 tokens, everything read from memory, called on a stream | inside a CUDA graph
+//                                        16.2 18.6 20.1 20.5 28.0 28.8 | 17.0 20.7 21.1 21.8 29.2 30.3
+//   the finish always before the heads   16.2 23.5 26.6 29.4 30.8 37.0 | 17.0 24.1 27.4 30.8 31.5 37.6
+//   the heads on a second stream         19.8 23.1 24.1 27.5 31.8 38.3 | 15.7 18.6 25.2 28.9 31.5 41.2
+// As a stage of the decode chain at 128 tokens: 24.5, 28.1 and 24.0.  Beyond two rounds every kernel fills the chip by itself
+// (1024 tokens: 45 us in the first order, 62 on two streams).
 struct IndexerPlan {
   bool finish_rows, finish_last;
   int proj_ctas, head_ctas;   // 0: one per SM
 };
 static IndexerPlan plan_indexer(int t) {
   const int sms = sm_count(), m_tiles = (t + 127) / 128, items = 64 * m_tiles, rounds = (items + sms - 1) / sms;
-  IndexerPlan pl{t > 192, false, 0, 0};
-  if (rounds > 2 || t + items <= sms) return pl;
+  if (rounds > 2 || t + items <= sms) return IndexerPlan{t > 192, false, 0, 0};
   const ProjPlan proj = proj_plan(t, 192, 7168 / 64);
-  pl.finish_rows = proj.m_tiles * proj.n_tiles * proj.splits + (t + 7) / 8 + items <= sms;
-  if (pl.finish_rows) return pl;
-  pl.finish_last = true;
-  pl.head_ctas = (items + rounds - 1) / rounds;
-  const int room = sms - pl.head_ctas, most = proj.m_tiles * proj.n_tiles * (10 / rounds);
-  pl.proj_ctas = room < most ? room : most;
-  return pl;
+  const int head_ctas = (items + rounds - 1) / rounds;
+  const int room = sms - head_ctas, most = proj.m_tiles * proj.n_tiles * (10 / rounds);
+  return IndexerPlan{false, true, room < most ? room : most, head_ctas};
 }
 
 // The V3.2 prologs: x times all weight matrices that take it (one launch), their finish (one), the heads (one).
