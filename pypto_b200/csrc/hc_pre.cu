@@ -25,7 +25,7 @@ namespace dsv32 {
 namespace {
 constexpr int kHc = 4, kHcD = 4096, kHcK = kHc * kHcD, kHcMix = (2 + kHc) * kHc, kHcOut = kHcMix + 1;
 constexpr int kHcSlice = 128, kHcSlices = kHcK / kHcSlice;   // 128 slices of 128 columns
-constexpr int kHcTokTile = 64, kHcDotThreads = 128, kHcFinThreads = 512;
+constexpr int kHcTokTile = 64, kHcDotThreads = 256, kHcFinThreads = 512;
 constexpr int kHcPad = kHcSlice + 4;                          // padded row stride of the shared-memory tiles
 constexpr size_t kHcDotSmem = static_cast<size_t>(kHcMix + kHcTokTile) * kHcPad * sizeof(float);   // 46,464 bytes
 
@@ -73,7 +73,8 @@ __device__ __forceinline__ uint4 hc_mix8(const uint4 (&x)[4], const float (&pre)
 }
 }  // namespace
 
-// One CTA per slice.  Dynamic shared memory:
+// One CTA per slice; all eight warps load, one per 16 tokens multiplies (with four warps the loads of 64 tokens were what the kernel
+// waited for: 18.5 us for the operator inside a graph, 14.0 now).  Dynamic shared memory:
 // w_s[24][132] (a slice of hc_fn, row stride padded so that the four output groups of a warp hit different banks)
 // and x_s[64][132] (the token tile's slice of x as floats, padded so that the eight token groups do).
 // Lane = (output group og = lane / 8: outputs 6 og .. 6 og + 5) x (token group tg = lane % 8: tokens tg, tg + 8 of
