@@ -189,7 +189,7 @@ size_t dsv32_scfa_workspace_bytes(int32_t t, int32_t topk, int32_t win_size) {
   if (t <= 0 || topk < 0 || win_size < 0) return 0;
   // cache row of every listed key, the length of every list, partial results of split lists (for the widest form)
   const int slots = scfa_slots(win_size, topk, 2);
-  const int splits = scfa_splits((t + 1) / 2, slots);   // (no call has fewer lists)
+  const int splits = scfa_most_splits((t + 1) / 2, slots);   // (no call has fewer lists)
   size_t bytes = align_up(static_cast<size_t>(t) * slots * sizeof(int32_t), 256) + align_up(static_cast<size_t>(t) * sizeof(int32_t), 256);
   if (splits > 1) bytes += align_up(static_cast<size_t>(t) * splits * 128 * (kKvLora + 1) * sizeof(float), 256);
   return bytes;
@@ -262,7 +262,8 @@ int dsv32_sparse_compress_attention(const Dsv32ScfaArgs* a, void* cuda_stream) {
   ws += align_up(static_cast<size_t>(a->t) * p.topk * sizeof(int32_t), 256);
   p.key_counts = reinterpret_cast<int32_t*>(ws);
   ws += align_up(static_cast<size_t>(a->t) * sizeof(int32_t), 256);
-  p.splits = scfa_splits(scfa_lists(a->t, a->b, p.pair), p.topk);
+  // (the selections of a pair mostly overlap: its list is taken as long as one of them)
+  p.splits = scfa_splits(scfa_lists(a->t, a->b, p.pair), p.topk, scfa_slots(a->win_size, a->topk, 1));
   p.part_o = reinterpret_cast<float*>(ws);
   p.part_lse = p.part_o + static_cast<size_t>(a->t) * p.splits * a->n_q * kKvLora;
   return launch_scfa_tc(p, static_cast<cudaStream_t>(cuda_stream));

@@ -83,7 +83,8 @@ int launch_sfa_tc(const SfaParams& p, cudaStream_t stream);
 int launch_sfa_combine(const SfaParams& p, cudaStream_t stream);
 int launch_scfa_tc(const SfaParams& p, cudaStream_t stream);   // the DeepSeek-V4 form (scfa_tc.cu)
 int scfa_lists(int t, int b, int pair);
-int scfa_splits(int lists, int slots);
+int scfa_most_splits(int lists, int slots);   // no call splits into more: what the workspace has room for
+int scfa_splits(int lists, int most_slots, int slots);   // slots: of a list as it is expected to be
 
 struct PrologParams {
   const __nv_bfloat16* x;

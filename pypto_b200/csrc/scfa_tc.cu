@@ -714,15 +714,32 @@ scfa_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
 // token, since the item of a second token, which has nothing to do, takes its turn like the others.
 int scfa_lists(int t, int b, int pair) { return pair && t % b == 0 && t / b % 2 == 0 ? t / 2 : t; }
 
-// Parts a key list is split into: while the items leave SMs idle, and no part below two tiles (a part costs its own Q, O and
-// a share of the combine kernel).  More items than CTAs would be a second round: 74 requests of one token, once counted as 37 pairs
-// and split in two, took 63.6 us with selected keys and 40.4 with ratio 128, unsplit 33.5 and 16.4; 20 requests of three tokens
-// 47.1 and 30.9, unsplit 32.8 and 16.5.
-int scfa_splits(int lists, int slots) {
+// Most parts a key list of `slots` entries is split into: while the items leave SMs idle, and no part below two tiles.  More items
+// than CTAs would be a second round: 74 requests of one token, once counted as 37 pairs and split in two, took 63.6 us with
+// selected keys and 40.4 with ratio 128, unsplit 33.5 and 16.4; 20 requests of three tokens 47.1 and 30.9, unsplit 32.8 and 16.5.
+int scfa_most_splits(int lists, int slots) {
   const int tiles = (slots + kScTile - 1) / kScTile;
   int s = sm_count() / (2 * (lists > 0 ? lists : 1));
   s = s < tiles / 2 ? s : tiles / 2;
   return s < 1 ? 1 : (s > 8 ? 8 : s);
+}
+// Of these the number that costs least: a tile takes about a microsecond, a split list the combine kernel and the partial results
+// of every part, about 4.5 and lists * parts / 12 of them.  us unsplit / in 2, 3, 4 and 8 parts (ctx 128K at ratio 128 is 24 tiles,
+// 64K 14, 8K 4, selected keys 14):
+//   ratio 128   1 list of 8K: 14.7 / 16.1 17.3   16 of 8K: 14.8 / 19.5 20.9   16 of 64K: 26.2 / 25.6 24.9 24.3
+//               1 of 128K: 36.3 / 27.6 23.6 21.2 18.8   16 of 128K: 37.1 / 31.3 28.7 26.7 26.8
+//   selected    1: 27.1 / 24.3 21.7 20.6 19.1   8: 29.4 / 27.1 25.0 24.1 26.2   32 pairs: 35.6 / 38.2
+int scfa_splits(int lists, int most_slots, int slots) {
+  const int most = scfa_most_splits(lists, most_slots), tiles = (slots + kScTile - 1) / kScTile;
+  int best = 1, best_cost = 12 * tiles;
+  for (int s = 2; s <= most; ++s) {
+    const int cost = 12 * tiles / s + 54 + lists * s;   // (not rounded to whole tiles: a list may be a tile longer than expected)
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
 }
 
 int launch_scfa_tc(const SfaParams& p, cudaStream_t stream) {
