@@ -4,7 +4,7 @@
 // checking two dozen tensors one by one in Python took longer (40-130 us a call) than the kernels ran.  Every function
 // here takes an entry point's tensors as they are, checks dtype, shape, contiguity and device against a short pattern,
 // takes the workspace from torch's caching allocator (stream-ordered, as torch.empty would), fills the argument block
-// and enqueues the operator on the current stream: 2-5 us plus the launches.  A call that does not fit its pattern -- a
+// and enqueues the operator on the current stream: 8-17 us a call with its two to four launches.  A call that does not fit its pattern -- a
 // wrong argument, a tensor on another device than the current one, a layout only the Python layer accepts -- is
 // declined (False / None) before anything is enqueued, and the Python layer, which knows every accepted form and every
 // error message, takes it from there.
